@@ -10,14 +10,18 @@
 // Tile: 16 keys.  S^T[16 keys, 8 columns] = K Q^T and O^T[HD, 8 columns] += V^T P^T, so the stored rows are the
 // 16-row operands as they lie in memory (V through transposing loads) and the query heads are the eight columns.
 // A warp's column fragments keep their lanes from S to O: maximum, sum and rescaling need no exchange but three
-// shuffles per tile.  P is not rounded to 16 bits: with at most four heads the columns past the heads carry the
-// rest p - round(p) of the same heads (their scores come from repeated query columns), and the two halves are added
-// at the end; eight heads take two products instead.  That is 17 bits of P in bf16, 22 in fp16, of weights at most 1.
+// shuffles per tile.  P keeps its 24 bits: three 16-bit pieces that add up to it.  The columns past the heads carry the
+// second (and, up to two heads, the third) piece of the same heads, whose scores come from repeated query columns; three and
+// four heads take two products, eight take three.  The pieces' sums are added at the end.  The unit cuts its sums off, which
+// over a long row of tiles would drift: a tile's products are added up on their own.  Error of the fp32 result against 64 bits
+// 2e-8 to 2e-7, as with fp32 FMAs (pieces of 17 bits: 2.5e-7 to 6e-7); its cost, us of 200 int8 sequences as above with 1 / 2 /
+// 4 / 8 heads a key: 99.9 / 99.6 / 99.9 / 71 -> 97.6 / 96.2 / 103.5 / 76, none in bf16.
 //
 // int8 pages: scores are exact integer products (mma .s8) with the query as two int8 terms per element,
 // q ~ qs (hi + lo / 128), 14 bits relative to the head's largest component.  Values become fp16 exactly (a byte under
-// 0x64 is 1024 + u); their row scale goes into the weight, divided by the largest scale seen so far so that the
-// weights use fp16's range.
+// 0x64 is 1024 + u; as bf16 they take two operations more: 118 us), so the pieces are fp16, of the weight times the row's
+// scale.  fp16's range suffices because the running reference that exponents are taken against is not the largest score but
+// the largest score + log2(scale): 2^14 times a weight is at most 2^14, and cut off at 2^-38 of the largest so far.
 //
 // Pipeline: 3 stages of 16 keys per warp, cp.async with zero fill past the last key (a zero weight must not meet
 // whatever the shared memory held), page-table entries one tile ahead of their copies.  bf16, 128 wide: 24 KB per
@@ -70,19 +74,42 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint
                : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// two values as 16-bit operands: rounded, or what the rounding leaves
+// First piece of a value: its upper half (eight bits) in bf16, rounded in fp16.  head2: of two values, packed.
+__device__ __forceinline__ float upper(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
 template <bool F16>
-__device__ __forceinline__ uint32_t pack_part(float a, float b, bool rest_a, bool rest_b) {
+__device__ __forceinline__ uint32_t head2(float a, float b) {
   if constexpr (F16) {
-    const __half ha = __float2half_rn(a), hb = __float2half_rn(b);
-    const __half2 p = __halves2half2(rest_a ? __float2half_rn(a - __half2float(ha)) : ha,
-                                     rest_b ? __float2half_rn(b - __half2float(hb)) : hb);
-    return *reinterpret_cast<const uint32_t*>(&p);
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
   } else {
-    const __nv_bfloat16 ha = __float2bfloat16_rn(a), hb = __float2bfloat16_rn(b);
-    const __nv_bfloat162 p = __halves2bfloat162(rest_a ? __float2bfloat16_rn(a - __bfloat162float(ha)) : ha,
-                                                rest_b ? __float2bfloat16_rn(b - __bfloat162float(hb)) : hb);
-    return *reinterpret_cast<const uint32_t*>(&p);
+    return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+  }
+}
+// what the first pieces leave of a, b
+template <bool F16>
+__device__ __forceinline__ float2 rest2(float a, float b) {
+  if constexpr (F16) {
+    const float2 h = __half22float2(__floats2half2_rn(a, b));
+    return make_float2(a - h.x, b - h.y);
+  } else {
+    return make_float2(a - upper(a), b - upper(b));
+  }
+}
+// o += a * (pieces).  fp16: a tile's products in one sum (one by one they cost 6 us of the above and gain nothing: the query's
+// 14 bits dominate).
+template <bool F16, int NP>
+__device__ __forceinline__ void add_product(float (&o)[4], const uint32_t (&a)[4], const uint32_t (&b)[NP][2]) {
+  constexpr int CHAIN = F16 ? NP : 1;
+#pragma unroll
+  for (int n0 = NP; n0 > 0; n0 -= CHAIN) {
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int n = n0 - 1; n >= n0 - CHAIN; --n) {
+      if constexpr (F16) mma_f16(sum, a, b[n][0], b[n][1]);
+      else mma_bf16(sum, a, b[n][0], b[n][1]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] += sum[j];
   }
 }
 
@@ -117,8 +144,8 @@ __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// q: [B, ldq] rows; part_o: fp32 [B, hq, splits, HD], part_ml: fp32 [B, hq, splits, 2] (running maximum in the log2
-// domain, sum); out (when not null: one split, no merge pass): [B, ldo] normalised rows.
+// q: [B, ldq] rows; part_o: fp32 [B, hq, splits, HD], part_ml: fp32 [B, hq, splits, 2] (the exponents' reference in the
+// log2 domain, sum); out (when not null: one split, no merge pass): [B, ldo] normalised rows.
 template <int HD, int G, bool I8, bool EXT>
 __global__ void __launch_bounds__(128, I8 ? 4 : 2)
 kernel(const __nv_bfloat16* __restrict__ q, int ldq, const uint8_t* __restrict__ kc, const uint8_t* __restrict__ vc,
@@ -126,7 +153,8 @@ kernel(const __nv_bfloat16* __restrict__ q, int ldq, const uint8_t* __restrict__
        const int* __restrict__ seqlens, float* __restrict__ part_o, float* __restrict__ part_ml,
        __nv_bfloat16* __restrict__ out, int ldo, int hq, int hk, int bs, int splits, float scale_log2, int gsplit, Ext x) {
   using C = Cfg<HD, I8>;
-  constexpr bool PAIRED = G <= 4;      // columns G .. 2G-1 repeat the heads and carry the rests of their weights
+  constexpr int PPP = 8 / G < 3 ? 8 / G : 3;    // pieces of the weights in a product: column c carries piece c / G of head c % G
+  constexpr int NP = (3 + PPP - 1) / PPP;       // products
   constexpr int MT = HD / 16;          // 16-row tiles of O^T
   constexpr int KS = I8 ? HD / 32 : HD / 16;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -149,9 +177,12 @@ kernel(const __nv_bfloat16* __restrict__ q, int ldq, const uint8_t* __restrict__
   float* scales = reinterpret_cast<float*>(smem + (C::PIPE > C::MERGE ? C::PIPE : C::MERGE)) + warp * C::NST * 32;
 
   // page row of this lane's key (lane & 15) of a tile, -1 past the last key
+  const uint32_t inverse = 0xffffffffu / (uint32_t)bs + 1;    // key / bs = key inverse / 2^32 while key bs < 2^32
+  const bool quick = bs > 1 && (uint64_t)max_blocks * bs * bs < (1ull << 32);
   auto page_row = [&](int tile) {
     const int key = k_begin + tile * 16 + (lane & 15);
-    return key < k_end ? (bt[key / bs] * hk + kvh) * bs + key % bs : -1;
+    const int page = quick ? (int)__umulhi((uint32_t)key, inverse) : key / bs;
+    return key < k_end ? (bt[page] * hk + kvh) * bs + key - page * bs : -1;
   };
   auto issue = [&](int stage, int my_row) {
     constexpr int RPP = 32 / C::CPR;   // rows per pass of the warp
@@ -222,9 +253,10 @@ kernel(const __nv_bfloat16* __restrict__ q, int ldq, const uint8_t* __restrict__
       for (int h = 0; h < 2; ++h) qb[0][s][h] = *reinterpret_cast<const uint32_t*>(qh + s * 16 + h * 8 + c0);
     col_scale[0] = col_scale[1] = scale_log2;
   }
-  const bool rest0 = PAIRED && c0 >= G, rest1 = PAIRED && c0 + 1 >= G;
+  // columns of second (third) pieces
+  const bool past1[2] = {c0 >= G, c0 + 1 >= G}, past2[2] = {c0 >= 2 * G, c0 + 1 >= 2 * G};
 
-  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, vmax = 0.f;
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
   float o[MT][4];
 #pragma unroll
   for (int t = 0; t < MT; ++t)
@@ -282,35 +314,33 @@ kernel(const __nv_bfloat16* __restrict__ q, int ldq, const uint8_t* __restrict__
     if (row >= left) sc[0] = sc[1] = -INFINITY;
     if (row + 8 >= left) sc[2] = sc[3] = -INFINITY;
 
-    float mt[2] = {fmaxf(sc[0], sc[2]), fmaxf(sc[1], sc[3])};
+    float mt[2], vscale[2];
+    if constexpr (I8) {
+      float up[2];                                      // log2 of a row's scale (rows of zeros: -100)
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        vscale[t] = scales[stage * 32 + 16 + row + 8 * t];
+        up[t] = fmaxf(__log2f(vscale[t]), -100.f);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) mt[j] = fmaxf(__fadd_ru(sc[j], up[0]), __fadd_ru(sc[j + 2], up[1]));   // no weight above 1
+    } else {
+      mt[0] = fmaxf(sc[0], sc[2]);
+      mt[1] = fmaxf(sc[1], sc[3]);
+    }
 #pragma unroll
     for (int d = 4; d <= 16; d <<= 1) {
       mt[0] = fmaxf(mt[0], __shfl_xor_sync(0xffffffffu, mt[0], d));
       mt[1] = fmaxf(mt[1], __shfl_xor_sync(0xffffffffu, mt[1], d));
     }
-    float w0 = 1.f, w1 = 1.f, alpha[2] = {1.f, 1.f};
-    bool grown = mt[0] > m[0] || mt[1] > m[1];
-    if constexpr (I8) {
-      const float v0 = scales[stage * 32 + 16 + row], v1 = scales[stage * 32 + 24 + row];
-      float v = fmaxf(v0, v1);
-#pragma unroll
-      for (int d = 4; d <= 16; d <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));
-      if (v > vmax) {                                   // the same in every lane
-        alpha[0] = alpha[1] = vmax / v;
-        vmax = v;
-        grown = true;
-      }
-      const float inv = vmax > 0.f ? 1.f / vmax : 0.f;
-      w0 = v0 * inv;
-      w1 = v1 * inv;
-    }
+    const bool grown = mt[0] > m[0] || mt[1] > m[1];
     if (__any_sync(0xffffffffu, grown)) {
+      float alpha[2];
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const float mm = fmaxf(m[j], mt[j]);
-        const float a = mm == -INFINITY ? 1.f : exp2f(m[j] - mm);   // every score so far -inf: nothing to rescale
-        l[j] *= a;
-        alpha[j] *= a;
+        alpha[j] = mm == -INFINITY ? 1.f : exp2f(m[j] - mm);   // every score so far -inf: nothing to rescale
+        l[j] *= alpha[j];
         m[j] = mm;
       }
 #pragma unroll
@@ -318,21 +348,38 @@ kernel(const __nv_bfloat16* __restrict__ q, int ldq, const uint8_t* __restrict__
 #pragma unroll
         for (int j = 0; j < 4; ++j) o[t][j] *= alpha[j & 1];
     }
-    float p[4];
+    // the weights' pieces as the column operand: keys 0..7, keys 8..15
+    uint32_t bw[NP][2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      p[j] = exp2f(sc[j] - m[j & 1]);
-      l[j & 1] += p[j];
-      p[j] *= j < 2 ? w0 : w1;
+    for (int t = 0; t < 2; ++t) {
+      float a = exp2f(sc[2 * t] - m[0]), b = exp2f(sc[2 * t + 1] - m[1]);
+      l[0] += a;
+      l[1] += b;
+      if constexpr (I8) {
+        a = a * vscale[t] * 16384.f;
+        b = b * vscale[t] * 16384.f;
+      }
+      const float2 r = rest2<I8>(a, b);
+      if constexpr (NP == 3) {
+        const float2 r2 = rest2<I8>(r.x, r.y);
+        bw[0][t] = head2<I8>(a, b);
+        bw[1][t] = head2<I8>(r.x, r.y);
+        bw[2][t] = head2<I8>(r2.x, r2.y);
+      } else if constexpr (NP == 2) {
+        const float2 r2 = rest2<I8>(r.x, r.y);
+        bw[0][t] = head2<I8>(past1[0] ? r.x : a, past1[1] ? r.y : b);
+        bw[1][t] = head2<I8>(past1[0] ? 0.f : r2.x, past1[1] ? 0.f : r2.y);
+      } else {
+        a = past1[0] ? r.x : a;
+        b = past1[1] ? r.y : b;
+        const float2 r2 = rest2<I8>(a, b);
+        bw[0][t] = head2<I8>(past2[0] ? r2.x : a, past2[1] ? r2.y : b);
+      }
     }
-    // weights as the column operand: keys 0..7, keys 8..15
-    const uint32_t b0 = transpose8x8(pack_part<I8>(p[0], p[1], rest0, rest1));
-    const uint32_t b1 = transpose8x8(pack_part<I8>(p[2], p[3], rest0, rest1));
-    uint32_t e0 = 0, e1 = 0;
-    if constexpr (!PAIRED) {
-      e0 = transpose8x8(pack_part<I8>(p[0], p[1], true, true));
-      e1 = transpose8x8(pack_part<I8>(p[2], p[3], true, true));
-    }
+#pragma unroll
+    for (int n = 0; n < NP; ++n)
+#pragma unroll
+      for (int t = 0; t < 2; ++t) bw[n][t] = transpose8x8(bw[n][t]);
     if constexpr (I8) {
       // rows r and r + 8 of a 16-row tile are dimensions 2 r and 2 r + 1: the transposing load moves byte pairs
 #pragma unroll
@@ -352,8 +399,7 @@ kernel(const __nv_bfloat16* __restrict__ q, int ldq, const uint8_t* __restrict__
             a[h * 2] = *reinterpret_cast<const uint32_t*>(&fe);
             a[h * 2 + 1] = *reinterpret_cast<const uint32_t*>(&fo);
           }
-          mma_f16(o[t + u], a, b0, b1);
-          if constexpr (!PAIRED) mma_f16(o[t + u], a, e0, e1);
+          add_product<I8>(o[t + u], a, bw);
         }
       }
     } else {
@@ -361,8 +407,7 @@ kernel(const __nv_bfloat16* __restrict__ q, int ldq, const uint8_t* __restrict__
       for (int t = 0; t < MT; ++t) {
         uint32_t a[4];
         ldsm4t(a, sv + C::at((lane & 7) + ((lane >> 4) << 3), t * 2 + ((lane >> 3) & 1)));
-        mma_bf16(o[t], a, b0, b1);
-        if constexpr (!PAIRED) mma_bf16(o[t], a, e0, e1);
+        add_product<I8>(o[t], a, bw);
       }
     }
     stage = stage + 1 == C::NST ? 0 : stage + 1;
@@ -381,13 +426,12 @@ kernel(const __nv_bfloat16* __restrict__ q, int ldq, const uint8_t* __restrict__
     s_l[warp][c0] = l[0];
     s_l[warp][c0 + 1] = l[1];
   }
-  const float ov = I8 ? vmax : 1.f;
 #pragma unroll
   for (int t = 0; t < MT; ++t)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int d = I8 ? t * 16 + row * 2 + (j >> 1) : t * 16 + row + (j >> 1) * 8;
-      s_o[(warp * 8 + c0 + (j & 1)) * HD + d] = o[t][j] * ov;
+      s_o[(warp * 8 + c0 + (j & 1)) * HD + d] = I8 ? o[t][j] * (1.f / 16384.f) : o[t][j];
     }
   __syncthreads();
   // one result per (head, dimension) of this split
@@ -407,7 +451,10 @@ kernel(const __nv_bfloat16* __restrict__ q, int ldq, const uint8_t* __restrict__
     for (int w = 0; w < 4; ++w) {
       const float a = s_m[w][g] == -INFINITY ? 0.f : exp2f(s_m[w][g] - mm);
       ll += s_l[w][g] * a;
-      oo += (s_o[(w * 8 + g) * HD + c] + (PAIRED ? s_o[(w * 8 + G + g) * HD + c] : 0.f)) * a;
+      float sum = 0.f;
+#pragma unroll
+      for (int k = PPP - 1; k >= 0; --k) sum += s_o[(w * 8 + k * G + g) * HD + c];
+      oo += sum * a;
     }
     if (merge) {
       kept[k] = oo;

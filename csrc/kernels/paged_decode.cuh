@@ -75,6 +75,8 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 // First piece of a value: its upper half (eight bits) in bf16, rounded in fp16.  head2: of two values, packed.
+// In bf16 all pieces of a weight are above 0, so that they make an infinite value's infinity and not its NaN: what is left
+// goes up by tiny(w), 2^-29 of the weight.  (fp16 pieces meet bytes.)
 __device__ __forceinline__ float upper(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
 template <bool F16>
 __device__ __forceinline__ uint32_t head2(float a, float b) {
@@ -85,14 +87,16 @@ __device__ __forceinline__ uint32_t head2(float a, float b) {
     return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
   }
 }
-// what the first pieces leave of a, b
 template <bool F16>
-__device__ __forceinline__ float2 rest2(float a, float b) {
+__device__ __forceinline__ float tiny(float w) { return F16 ? 0.f : fmaxf(w * 0x1p-29f, 0x1p-126f); }
+// what the first pieces leave of a, b; ta, tb: tiny of the weights
+template <bool F16>
+__device__ __forceinline__ float2 rest2(float a, float b, float ta, float tb) {
   if constexpr (F16) {
     const float2 h = __half22float2(__floats2half2_rn(a, b));
     return make_float2(a - h.x, b - h.y);
   } else {
-    return make_float2(a - upper(a), b - upper(b));
+    return make_float2(a - upper(a) + ta, b - upper(b) + tb);
   }
 }
 // o += a * (pieces).  fp16: a tile's products in one sum (one by one they cost 6 us of the above and gain nothing: the query's
@@ -359,20 +363,21 @@ kernel(const __nv_bfloat16* __restrict__ q, int ldq, const uint8_t* __restrict__
         a = a * vscale[t] * 16384.f;
         b = b * vscale[t] * 16384.f;
       }
-      const float2 r = rest2<I8>(a, b);
+      const float ta = tiny<I8>(a), tb = tiny<I8>(b);
+      const float2 r = rest2<I8>(a, b, ta, tb);
       if constexpr (NP == 3) {
-        const float2 r2 = rest2<I8>(r.x, r.y);
+        const float2 r2 = rest2<I8>(r.x, r.y, ta, tb);
         bw[0][t] = head2<I8>(a, b);
         bw[1][t] = head2<I8>(r.x, r.y);
         bw[2][t] = head2<I8>(r2.x, r2.y);
       } else if constexpr (NP == 2) {
-        const float2 r2 = rest2<I8>(r.x, r.y);
+        const float2 r2 = rest2<I8>(r.x, r.y, ta, tb);
         bw[0][t] = head2<I8>(past1[0] ? r.x : a, past1[1] ? r.y : b);
-        bw[1][t] = head2<I8>(past1[0] ? 0.f : r2.x, past1[1] ? 0.f : r2.y);
+        bw[1][t] = head2<I8>(past1[0] ? ta : r2.x, past1[1] ? tb : r2.y);
       } else {
         a = past1[0] ? r.x : a;
         b = past1[1] ? r.y : b;
-        const float2 r2 = rest2<I8>(a, b);
+        const float2 r2 = rest2<I8>(a, b, ta, tb);
         bw[0][t] = head2<I8>(past2[0] ? r2.x : a, past2[1] ? r2.y : b);
       }
     }

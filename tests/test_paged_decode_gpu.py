@@ -140,3 +140,22 @@ def test_small_values_beside_a_large_one_without_weight(hd, ratio):
     s = torch.einsum("hd,shd->hs", q[-1].double().reshape(hq, hd), k.repeat_interleave(ratio, 1)) * hd ** -0.5
     want = torch.einsum("hs,shd->hd", torch.softmax(s, -1), v.repeat_interleave(ratio, 1)).reshape(-1)
     assert float((out[-1].double() - want).norm() / want.norm()) < 2 ** -9 + 2e-3      # as for every int8 page
+
+
+@pytest.mark.parametrize("hd,ratio", [(128, 1), (128, 2), (128, 4), (128, 8), (64, 3)])
+@pytest.mark.parametrize("splits", [1, 3, 9])
+def test_an_infinite_value_stays_infinite(hd, ratio, splits):
+    """A weighted sum with an infinity in it is that infinity, whatever the weight's bits; other columns do not see it."""
+    hk, bs = 2, 16
+    hq = hk * ratio
+    _, tables, q, pools, scales, n, want = _case(hq, hk, hd, bs, False)
+    want = want.clone()
+    for b, length in enumerate(LENS):
+        for at, col, value in ((0, 5, math.inf), (length - 1, 40, -math.inf)):
+            pools[1][tables[b, at // bs].long(), :, at % bs, col] = value
+            want.reshape(len(LENS), hq, hd)[b, :, col] = value
+    out, _, _ = _run(False, tables, q, pools, scales, n, hq, hk, hd, bs, splits)
+    finite = torch.isfinite(want)
+    assert torch.equal(out.double()[~finite], want[~finite])
+    err = torch.where(finite, out.double() - want, 0.0).norm() / torch.where(finite, want, 0.0).norm()
+    assert float(err) < 2 ** -9 + 2 ** -14

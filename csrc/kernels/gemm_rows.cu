@@ -53,6 +53,7 @@ __device__ __forceinline__ uint4 ld_peer_u4(uint32_t addr) {
   return v;
 }
 __device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();   // .aligned wants whole warps: the loops in front of it may end in the middle of one
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

@@ -144,6 +144,7 @@ __device__ __forceinline__ float ld_peer(uint32_t local, uint32_t rank) {
   return v;
 }
 __device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();   // .aligned wants whole warps
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

@@ -298,12 +298,10 @@ int launch(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const Args& a, int 
   return (int)cudaLaunchKernelEx(&cfg, kernel<I8, GLU>, tm_w, tm_x, a);
 }
 
-template <bool I8>
-int run(const void* A, const void* B, Args a, int K, int lda, int ldb, int slices, int smem_kb, cudaStream_t stream) {
-  constexpr int ES = I8 ? 1 : 2, BK = I8 ? 128 : 64;
-  const CUtensorMapDataType dt = I8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+// Fills in the ring, the slices that are left of `slices`, and the columns of tensor memory; *smem = shared memory of a CTA.
+int plan(Args& a, int K, int bk, int slices, int smem_kb, int* smem) {
   a.rows_pad = (a.M + 15) / 16 * 16;
-  a.nkb = (K + BK - 1) / BK;
+  a.nkb = (K + bk - 1) / bk;
   a.kb_per = (a.nkb + slices - 1) / slices;
   a.slices = (a.nkb + a.kb_per - 1) / a.kb_per;
   a.stage_bytes = W_BYTES + a.rows_pad * KB;
@@ -317,12 +315,27 @@ int run(const void* A, const void* B, Args a, int K, int lda, int ldb, int slice
   a.rows_part = ring / (16 * BN * 4) * 16;
   a.tmem_cols = 32;
   while (a.tmem_cols < a.rows_pad) a.tmem_cols *= 2;
+  // A CTA takes at least the share of the SM's shared memory (228 KB, 1 KB of it for each CTA) that its columns are of tensor
+  // memory: CTAs that share an SM, other launches' among them, then never ask for more than its 512 columns.  One that waited
+  // for columns while its cluster waits for it could wait for a cluster that waits for columns here.
+  const int share = a.tmem_cols * (228 * 1024 / 512) - 1024;
+  *smem = 1024 + BAR_BYTES + ring;
+  if (*smem < share) *smem = share;
+  return BB_OK;
+}
+
+template <bool I8>
+int run(const void* A, const void* B, Args a, int K, int lda, int ldb, int slices, int smem_kb, cudaStream_t stream) {
+  constexpr int ES = I8 ? 1 : 2, BK = I8 ? 128 : 64;
+  const CUtensorMapDataType dt = I8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  int smem;
+  int rc = plan(a, K, BK, slices, smem_kb, &smem);
+  if (rc) return rc;
   CUtensorMap tm_w, tm_x;
-  int rc = make_tmap_2d(&tm_w, dt, ES, B, K, a.ff ? 2 * a.ff : a.N, (uint64_t)ldb * ES, BK, a.ff ? BN / 2 : BN);
+  rc = make_tmap_2d(&tm_w, dt, ES, B, K, a.ff ? 2 * a.ff : a.N, (uint64_t)ldb * ES, BK, a.ff ? BN / 2 : BN);
   if (rc) return rc;
   rc = make_tmap_2d(&tm_x, dt, ES, A, K, a.M, (uint64_t)lda * ES, BK, a.rows_pad);
   if (rc) return rc;
-  const int smem = 1024 + BAR_BYTES + ring;
   return a.ff ? launch<I8, true>(tm_w, tm_x, a, smem, stream) : launch<I8, false>(tm_w, tm_x, a, smem, stream);
 }
 
@@ -400,6 +413,21 @@ BB_API int bb_gemm_rows(const void* A, const void* B, void* C, const float* bias
                         int M, int N, int K, int lda, int ldb, int ldc, int i8, int out_mode, float alpha, int slices,
                         int smem_kb, int early, void* stream) {
   return gemm_rows(A, B, C, bias, scale_m, scale_n, M, N, K, lda, ldb, ldc, i8, out_mode, alpha, slices, smem_kb, early, 0, stream);
+}
+
+// How gemm_rows would launch these sizes on `sms` SMs: out = slices, bytes of shared memory and columns of tensor memory of a
+// CTA.  No device is needed.
+BB_API int bb_gemm_rows_plan(int M, int N, int K, int i8, int ff, int sms, int slices, int smem_kb, int* out) {
+  if (M <= 0 || N <= 0 || K <= 0 || M > 256) return BB_ESIZE;
+  rows::Args a{};
+  a.M = M;
+  const int bk = i8 ? 128 : 64, per = ff ? rows::BN / 2 : rows::BN;
+  if (slices == 0) rows::split(M, (N + per - 1) / per, (K + bk - 1) / bk, sms, &slices, &smem_kb);
+  if (slices < 1 || slices > 8 || smem_kb < 32 || smem_kb > 226) return BB_EARG;
+  const int rc = rows::plan(a, K, bk, slices, smem_kb, &out[1]);
+  out[0] = a.slices;
+  out[2] = a.tmem_cols;
+  return rc;
 }
 
 // C[M, ff] bf16 = silu(A G^T) * (A U^T) for B = [G; U] of ff rows each: a tile is 64 gate and the 64 matching up channels,

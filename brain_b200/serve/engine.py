@@ -220,9 +220,17 @@ class QwenEngine(PagedEngineBase):
         blk = torch.gather(block_table, 1, (positions // bs).long()[:, None]).squeeze(1)
         return (blk * bs + positions % bs).to(torch.int32)
 
+    def _check_positions(self, positions: np.ndarray, tables: np.ndarray, window: int = 1) -> None:
+        """Refuses positions that steps of ``window`` tokens would look up outside the block tables: the kernels do not check."""
+        p = np.asarray(positions)
+        if p.size and (int(p.min()) < 0 or int(p.max()) + window > np.shape(tables)[-1] * self.block_size):
+            raise IndexError(f"positions {int(p.min())}..{int(p.max()) + window - 1} in tables of {np.shape(tables)[-1]} blocks "
+                             f"of {self.block_size}")
+
     def _slots_host(self, block_table: np.ndarray, positions: np.ndarray) -> np.ndarray:
         """The same for one sequence's host table."""
         bs = self.block_size
+        self._check_positions(positions, block_table)
         return np.asarray(block_table, dtype=np.int32)[positions // bs] * bs + positions % bs
 
     def _upload(self, *arrays):
@@ -586,6 +594,7 @@ class QwenEngine(PagedEngineBase):
         block_tables = np.asarray(block_tables, dtype=np.int32)
         pos_np = [np.arange(it[1], it[1] + l, dtype=np.int32) for it, l in zip(items, lens)]
         # the rows that sample: last row of each finishing prompt + decode rows
+        self._check_positions(positions, block_tables)
         final = [i for i, it in enumerate(items) if it[3]]
         tok, pos, slots, dlens, rows, dbts, *bts = self._upload(
             np.concatenate([np.asarray(it[0], dtype=np.int32) for it in items] + [np.asarray(tokens, dtype=np.int32)]),
@@ -635,6 +644,10 @@ class QwenEngine(PagedEngineBase):
 
     def _decode_steps(self, tok, pos, bts, window: int, greedy: bool, slots=None):
         """``window`` decode steps on device tensors -> (tokens [B, window], last top-k or None)."""
+    def _decode(self, tokens, positions, block_tables, window, greedy, slots):
+        self._check_positions(positions, block_tables, window)
+        return super()._decode(tokens, positions, block_tables, window, greedy, slots)
+
         B = tok.shape[0]
         outs = []
         topks = None

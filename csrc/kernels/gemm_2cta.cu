@@ -493,9 +493,43 @@ BB_API int bb_gemm_pair_set_debug(long long* buf) {
 }
 #endif
 
-// Number of 2-CTA clusters the current device runs at once, as found by the first launch (0 before).
-static std::atomic<int> g_last_pairs_fit{0};
-BB_API int bb_gemm_pair_clusters() { return g_last_pairs_fit.load(); }
+// Number of 2-CTA clusters the current device runs at once (an odd SM count per GPC leaves one SM out).  Asked of the device on
+// its first use, so that every product of a process is planned with the same number.  All forms of the kernel take an SM per
+// CTA: one answers for all.
+BB_API int bb_gemm_pair_clusters() {
+  using namespace bb;
+  using namespace bb::pair;
+  static const int forced = [] {
+    const char* e = getenv("BB_PAIR_CLUSTERS");
+    return e ? atoi(e) : 0;
+  }();
+  if (forced > 0) return forced;
+  static std::atomic<int> max_pairs[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const bool keep = dev >= 0 && dev < 64;
+  int n = keep ? max_pairs[dev].load(std::memory_order_relaxed) : 0;
+  if (n > 0) return n;
+  static PerDeviceOnce once;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2 * (sm_count() / 2));
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = SMEM;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (ensure_dyn_smem(once, gemm_pair_kernel<false, false>, SMEM) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<false, false>, &cfg) != cudaSuccess || n <= 0) {
+    cudaGetLastError();
+    n = sm_count() / 2 - 2;
+  }
+  if (keep) max_pairs[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
 
 // Pair-tile bf16 GEMM (see the top of the file).  Same argument meaning as bb_gemm_bf16; serves
 // out_mode 0 / 1 / 2 (bias: modes 0 and 1).  Returns BB_ESIZE when the shape or alignment does not suit the
@@ -530,39 +564,7 @@ static int launch_pair(const void* A, const void* B, void* C, const float* bias,
     cudaError_t e = ensure_dyn_smem(smem_once, gemm_pair_kernel<I8, GLU>, SMEM);
     if (e != cudaSuccess) return (int)e;
   }
-  // how many 2-CTA clusters the device holds at once (an odd SM count per GPC leaves one SM out)
-  static std::atomic<int> max_pairs[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int pairs_fit = (dev >= 0 && dev < 64) ? max_pairs[dev].load(std::memory_order_relaxed) : 0;
-  if (pairs_fit == 0) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(2 * (sm_count() / 2));
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = SMEM;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<I8, GLU>, &cfg) != cudaSuccess || n <= 0) {
-      cudaGetLastError();
-      n = sm_count() / 2 - 2;
-    }
-    pairs_fit = n;
-    if (dev >= 0 && dev < 64) max_pairs[dev].store(n, std::memory_order_relaxed);
-  }
-  {
-    static const int forced = [] {
-      const char* e = getenv("BB_PAIR_CLUSTERS");
-      return e ? atoi(e) : 0;
-    }();
-    if (forced > 0) pairs_fit = forced;
-  }
-  g_last_pairs_fit.store(pairs_fit);
+  const int pairs_fit = bb_gemm_pair_clusters();
   PairArgs a{};
   a.bias = bias;
   a.ff = GLU ? N : 0;

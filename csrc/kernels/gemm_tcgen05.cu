@@ -946,8 +946,7 @@ struct GemmPick {
 // 12288 59 / 41, 560 x 4096 x 4096 23.7 / 17.5.
 GemmPick pick_gemm(bool i8, int M, int N, int nkb, bool add, bool split, bool pair_ok, int max_ctas) {
   const int ctas = max_ctas > 0 ? max_ctas : bb::sm_count();
-  const int fit = bb_gemm_pair_clusters();
-  const int pairs = max_ctas > 0 ? max_ctas / 2 : (fit > 0 ? fit : bb::sm_count() / 2);
+  const int pairs = max_ctas > 0 ? max_ctas / 2 : bb_gemm_pair_clusters();
   GemmPick best{64, 1, false};
   double best_us = 1e30;
   for (const GemmForm& f : FORMS[i8]) {

@@ -124,3 +124,25 @@ def test_pair_glu_is_the_product_and_its_activation(M, ff, K, int8):
     assert lib.bb_swiglu_fwd(_p(gu), _p(want), C.c_long(M), ff, _stream()) == 0
     _cuda.check_error()
     assert torch.equal(got[:, :ff], want) and bool((got[:, ff:] == 7.0).all())
+
+
+def test_products_are_planned_alike_from_the_first_on():
+    """The number of CTA pairs that forms are chosen by is the device's, in a process that has launched none and after it."""
+    import subprocess
+    import sys
+    code = """
+import ctypes as C, torch
+from brain_b200.ops import _cuda
+lib = _cuda.lib()
+a = torch.zeros(256, 256, device="cuda", dtype=torch.int8)
+one = torch.ones(256, device="cuda")
+out = torch.empty(256, 256, device="cuda", dtype=torch.bfloat16)
+before = lib.bb_gemm_pair_clusters()
+p = lambda t: C.c_void_p(t.data_ptr())
+assert lib.bb_gemm_i8_pair(p(a), p(a), p(out), p(one), p(one), 256, 256, 256, 256, 256, 256, 0, None) == 0
+torch.cuda.synchronize()
+assert 0 < before == lib.bb_gemm_pair_clusters(), (before, lib.bb_gemm_pair_clusters())
+print("pairs", before)
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr

@@ -27,6 +27,7 @@ def fused_ok(x, params) -> bool:
 def _project(x, w, bias, n, s):
     """x [n, k] @ w [m, k]^T (+ bias)"""
     m, k = w.shape
+    assert x.shape == (n, k) and w.stride(1) == 1, (x.shape, w.shape, w.stride())
     y = torch.empty(n, m, device=x.device, dtype=torch.bfloat16)
     call("gemm_bf16", x, w, y, bias, n, m, k, k, w.stride(0), m, 0, 0, 0, 1.0, 0, 0, s)
     return y
@@ -35,9 +36,11 @@ def _project(x, w, bias, n, s):
 def _project_back(dy, x, w, wp, bp, n, s):
     """Gradient of _project: adds into the parameters' main_grad, returns dx."""
     m, k = w.shape
+    mg = wp.main_grad
+    assert dy.shape == (n, m) and x.shape == (n, k), (dy.shape, x.shape, w.shape)
+    assert mg.shape == w.shape and mg.stride(1) == 1 and mg.dtype == torch.float32, (mg.shape, mg.stride(), mg.dtype)
     dx = torch.empty(n, k, device=dy.device, dtype=torch.bfloat16)
     call("gemm_bf16", dy, w, dx, None, n, k, m, m, w.stride(0), k, 0, 1, 0, 1.0, 0, 0, s)
-    mg = wp.main_grad
     call("gemm_bf16", dy, x, mg, None, m, k, n, m, k, mg.stride(0), 1, 1, 2, 1.0, 0, 0, s)
     F._notify(wp)
     if bp is not None:

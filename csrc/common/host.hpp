@@ -57,6 +57,12 @@ inline cudaError_t ensure_dyn_smem(PerDeviceOnce& once, K kernel, int bytes) {
   return e;
 }
 
+// A launch's own result, taken off the runtime's last error, which the next launch to ask (torch's too) would take for its own.
+inline int launched(cudaError_t e) {
+  if (e != cudaSuccess) cudaGetLastError();
+  return (int)e;
+}
+
 // Launch that may overlap the end of the kernel before it on the stream: the launch and the prologue of a decode step's
 // 2 to 10 us kernels otherwise cost about as much as they do.  The kernel calls pdl_wait (ptx.cuh).
 template <typename... P, typename... A>
@@ -71,7 +77,7 @@ inline int launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   cfg.stream = stream;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return launched(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
 int* device_error_word();  // per-device int, zero-initialised, lives until exit

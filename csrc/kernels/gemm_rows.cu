@@ -295,7 +295,7 @@ int launch(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const Args& a, int 
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  return (int)cudaLaunchKernelEx(&cfg, kernel<I8, GLU>, tm_w, tm_x, a);
+  return launched(cudaLaunchKernelEx(&cfg, kernel<I8, GLU>, tm_w, tm_x, a));
 }
 
 // Fills in the ring, the slices that are left of `slices`, and the columns of tensor memory; *smem = shared memory of a CTA.

@@ -544,9 +544,9 @@ static int launch_pdec(dim3 grid, cudaStream_t s, const void* q, int ldq, const 
   cfg.stream = s;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  return (int)cudaLaunchKernelEx(&cfg, pdec::kernel<HD, G, I8, EXT>, (const __nv_bfloat16*)q, ldq, (const uint8_t*)kc, (const uint8_t*)vc, ks, vs,
+  return launched(cudaLaunchKernelEx(&cfg, pdec::kernel<HD, G, I8, EXT>, (const __nv_bfloat16*)q, ldq, (const uint8_t*)kc, (const uint8_t*)vc, ks, vs,
                                                           block_tables, max_blocks, seqlens, part_o, part_ml, (__nv_bfloat16*)out, ldo,
-                                                          hq, hk, bs, splits, sl2, gsplit, x);
+                                                          hq, hk, bs, splits, sl2, gsplit, x));
 }
 
 static int launch_paged_decode(bool i8, const void* q, int ldq, const void* kc, const void* vc,

@@ -289,3 +289,17 @@ def test_w4a8_unpack_kernel_and_engine():
     g2, _ = e4.decode(nxt, pos, bt[None, :], greedy=True)
     assert g1 == g2
     _cuda.check_error()
+
+
+def test_a_refused_launch_is_not_reported_by_the_next():
+    """More splits than a grid is deep: an error of the launch call, and of no later one's."""
+    from brain_b200.ops._cuda import NativeError, call, check_error, stream_ptr
+    kc = torch.zeros(2, 1, 16, 64, device="cuda", dtype=torch.bfloat16)
+    q = torch.zeros(1, 64, device="cuda", dtype=torch.bfloat16)
+    table, one = (torch.ones(s, device="cuda", dtype=torch.int32) for s in ((1, 1), (1,)))
+    part = torch.zeros(80000 * 64, device="cuda")
+    with pytest.raises(NativeError):
+        call("paged_decode", q, 64, kc, kc, table, 1, one, q, 64, part, part, 1, 1, 1, 64, 16, 70000, 0.125, stream_ptr())
+    call("kv_append", q, 64, q, 64, one, kc, kc, 1, 1, 64, 16, stream_ptr())
+    assert float((q + 1).sum()) == 64.0
+    check_error()

@@ -7,7 +7,6 @@ A subclass provides ``_decode_steps(tok, pos, bts, window, greedy, slots)`` over
 recurrent state also set ``state_slots`` (slots the scheduler hands out) and ``dummy_slot``."""
 from __future__ import annotations
 
-import gc
 import time
 
 import numpy as np
@@ -154,16 +153,8 @@ class PagedEngineBase:
         graph = torch.cuda.CUDAGraph()
         # thread-local capture mode: other threads of the process (e.g. a process group's watchdog)
         # keep making CUDA calls of their own while this thread captures
-        # no garbage collection meanwhile: what it frees (another engine's graph, pinned memory) may be a call that a
-        # capturing thread must not make
-        collecting = gc.isenabled()
-        gc.disable()
-        try:
-            with torch.cuda.graph(graph, capture_error_mode="thread_local"):
-                out, _ = self._decode_steps(g["tok"], g["pos"], g["bts"], window, True, slot)
-        finally:
-            if collecting:
-                gc.enable()
+        with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+            out, _ = self._decode_steps(g["tok"], g["pos"], g["bts"], window, True, slot)
         g["graph"], g["out"] = graph, out
         self.steps = steps0
         return g

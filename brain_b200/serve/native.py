@@ -5,6 +5,7 @@ prefill, and ``decode`` for a whole decode step."""
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 from typing import Dict, Optional
 
 import torch
@@ -91,7 +92,7 @@ class NativeForward:
         return True
 
     def __init__(self, eng):
-        self.eng = eng
+        self.eng = weakref.proxy(eng)     # an engine that nobody holds goes at once, with its graphs and pools
         self.lib = _cuda.lib()
         n = len(eng.layers)
         self._layers = (Layer * n)()

@@ -1,4 +1,7 @@
-"""What a serving engine refuses before any work is issued (CPU)."""
+"""What a serving engine refuses before any work is issued, and its small host-side pieces (CPU)."""
+import gc
+import weakref
+
 import numpy as np
 import pytest
 
@@ -37,3 +40,19 @@ def test_the_last_position_of_a_table_is_served():
     tables = np.arange(8, dtype=np.int32)[None, :]
     toks, _ = eng.decode(np.array([1], dtype=np.int32), np.array([62], dtype=np.int32), tables, window=2)
     assert len(toks[0]) == 2
+
+
+def test_an_engine_goes_with_its_last_reference():
+    """Also one with the native forward: what waits for a collection may be freed while another engine's step is captured."""
+    from brain_b200.serve.native import NativeForward
+    eng = _engine()
+    eng.native = NativeForward(eng)
+    gone = weakref.ref(eng)
+    collecting = gc.isenabled()
+    gc.disable()
+    try:
+        del eng
+        assert gone() is None
+    finally:
+        if collecting:
+            gc.enable()

@@ -303,3 +303,51 @@ def test_a_refused_launch_is_not_reported_by_the_next():
     call("kv_append", q, 64, q, 64, one, kc, kc, 1, 1, 64, 16, stream_ptr())
     assert float((q + 1).sum()) == 64.0
     check_error()
+
+
+def test_engines_go_with_their_last_reference():
+    """With their captured steps: what waits for a collection may be freed while another engine's step is captured."""
+    import gc
+    import os
+    import sys
+    import weakref
+    sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+    import hybrid_util
+    collecting = gc.isenabled()
+    gc.collect()
+    gc.disable()
+    try:
+        engines = [_engine(), hybrid_util.engine(hybrid_util.mixed_model()[0], "bf16")]
+        for eng in engines:
+            kw = {"slots": np.array([0], dtype=np.int32)} if eng.state_slots else {}
+            eng.decode(np.array([3], dtype=np.int32), np.array([0], dtype=np.int32), np.arange(eng.max_blocks, dtype=np.int32)[None, :], **kw)
+            assert eng._graphs
+        gone = [weakref.ref(e) for e in engines]
+        del engines, eng
+        assert [g() for g in gone] == [None, None]
+    finally:
+        if collecting:
+            gc.enable()
+
+
+def test_a_capture_leaves_garbage_collection_as_it_is():
+    """Another thread's switch is not touched, in the capture or behind it."""
+    import gc
+    eng = _engine()
+    steps, seen = eng._decode_steps, []
+
+    def watched(*a, **kw):
+        seen.append((torch.cuda.is_current_stream_capturing(), gc.isenabled()))
+        return steps(*a, **kw)
+
+    eng._decode_steps = watched
+    collecting = gc.isenabled()
+    try:
+        for want in (True, False):
+            gc.enable() if want else gc.disable()
+            eng._graphs.clear()
+            seen.clear()
+            eng.decode(np.array([3], dtype=np.int32), np.array([0], dtype=np.int32), np.arange(eng.max_blocks, dtype=np.int32)[None, :])
+            assert (True, want) in seen and all(on == want for _, on in seen) and gc.isenabled() == want
+    finally:
+        gc.enable() if collecting else gc.disable()

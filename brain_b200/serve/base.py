@@ -21,8 +21,8 @@ def read_back(tokens, topk):
     if topk is None:
         return tokens.cpu().tolist(), None
     ids, logits = topk
-    k = ids.shape[-1]
-    flat = torch.cat([tokens.reshape(ids.shape[0], -1).to(torch.int32), ids.to(torch.int32), logits.float().view(torch.int32)], 1).cpu().numpy()
+    n, k = ids.shape
+    flat = torch.cat([tokens.reshape(n, tokens.shape[1] if tokens.dim() > 1 else 1).to(torch.int32), ids.to(torch.int32), logits.float().view(torch.int32)], 1).cpu().numpy()
     picked = flat[:, :-2 * k]
     cands = [list(zip(i, v)) for i, v in zip(flat[:, -2 * k:-k].tolist(), np.ascontiguousarray(flat[:, -k:]).view(np.float32).tolist())]
     return picked.reshape(tokens.shape).tolist(), cands

@@ -4,9 +4,11 @@ import weakref
 
 import numpy as np
 import pytest
+import torch
 
 from brain_b200.models.config import QwenConfig
 from brain_b200.models.qwen3 import Qwen3
+from brain_b200.serve.base import read_back
 from brain_b200.serve.engine import QwenEngine
 
 
@@ -40,6 +42,18 @@ def test_the_last_position_of_a_table_is_served():
     tables = np.arange(8, dtype=np.int32)[None, :]
     toks, _ = eng.decode(np.array([1], dtype=np.int32), np.array([62], dtype=np.int32), tables, window=2)
     assert len(toks[0]) == 2
+
+
+@pytest.mark.parametrize("shape", [(0,), (0, 2), (3,), (3, 1), (3, 4)])
+def test_read_back_of_tokens_and_candidates(shape):
+    g = torch.Generator().manual_seed(1)
+    tokens = torch.randint(0, 1 << 30, shape, generator=g, dtype=torch.int32)
+    ids = torch.randint(0, 1 << 30, (shape[0], 5), generator=g, dtype=torch.int32)
+    logits = torch.randn(shape[0], 5, generator=g)
+    picked, cands = read_back(tokens, (ids, logits))
+    assert picked == tokens.tolist()
+    assert cands == [list(zip(i, v)) for i, v in zip(ids.tolist(), logits.tolist())]
+    assert read_back(tokens, None) == (tokens.tolist(), None)
 
 
 def test_an_engine_goes_with_its_last_reference():

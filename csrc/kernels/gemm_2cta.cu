@@ -159,7 +159,8 @@ __device__ __forceinline__ void add_bias32(float (&v)[32], const float* __restri
 
 // GLU: the leader stages 128 gate rows of B and the peer the matching up rows, so columns c and c + 128 of an accumulator row
 // belong together and the epilogue stores silu(gate) * up, both rounded to bf16 before, as [M, ff]: the [M, 2 ff] product is
-// not written and read again (prompts of 8192 x 6144 x 2048: 270 us and 49 for SwiGLU; in one kernel 276).
+// not written and read again (prompts of 8192 x 6144 x 2048: 270 us and 49 for SwiGLU; in one kernel 276).  Its epilogue reads
+// two accumulators a column: where it pays is glu_on_pairs' (gemm_tcgen05.cu) to say.
 template <bool I8, bool GLU>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,

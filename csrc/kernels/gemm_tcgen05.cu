@@ -966,6 +966,36 @@ GemmPick pick_gemm(bool i8, int M, int N, int nkb, bool add, bool split, bool pa
   return best;
 }
 
+// Whether gate, up and SwiGLU run faster as one kernel on CTA pairs than as the product [M, 2 ff] in the form that pick_gemm
+// chooses and a pass over it: fewer bytes, but 256 x 128 tiles whose epilogue (two accumulators, exp) takes 4 to 8 us, and for
+// int8 rows another pass behind it.  us of a tile: its k-blocks or its epilogue, the longer (they overlap); fits to 230 pairs of
+// sizes a type (256 to 8192 rows, ff 256 to 17408, K 256 to 5120): 0.1 % (bf16) and 0.3 % (int8) slower in the mean than the
+// faster form at each size, 6 and 11 % at the worst; one kernel always is 8 and 23 % in the mean.  us, apart / one kernel:
+// 8192 x 6144 x 2048 375 / 341, 2200 x 3072 x 1024 31 / 26, 300 x 6144 x 2048 25.6 / 39, 512 x 512 x 512 8.2 / 10.7;
+// int8 8192 x 12288 x 4096 703 / 650, 1072 x 3072 x 1024 21.8 / 24.5, 1072 x 6144 x 2048 39 / 45, 512 x 512 x 512 8.1 / 13.9.
+struct TileTime {
+  double per_block, epilogue, fixed;
+  double us(long tiles, long slots, int nkb) const {
+    const double tile = nkb * per_block;
+    return (double)((tiles + slots - 1) / slots) * (tile > epilogue ? tile : epilogue) + fixed;
+  }
+};
+constexpr TileTime PRODUCT[2][4] = {{{0.25, 0.0, 4.5}, {0.28, 0.0, 5.0}, {0.44, 2.5, 5.0}, {0.42, 4.25, 4.0}},    // as FORMS
+                                    {{0.27, 0.0, 5.0}, {0.33, 1.5, 5.5}, {0.45, 4.5, 6.0}, {0.40, 5.25, 7.0}}};
+constexpr TileTime PAIR_GLU[2] = {{0.40, 4.25, 7.5}, {0.43, 8.0, 7.0}};
+
+bool glu_on_pairs(bool i8, int M, int ff, int K) {
+  if (!pair_enabled() || M < 256 || ff < 256 || K < 256) return false;
+  const int bk = i8 ? 128 : 64, nkb = (K + bk - 1) / bk, pairs = bb_gemm_pair_clusters();
+  const GemmPick p = pick_gemm(i8, M, 2 * ff, nkb, false, false, true, 0);
+  const int form = p.pair ? 3 : (p.bn == 64 ? 0 : p.bn == 128 ? 1 : 2), rows = p.pair ? 256 : 128, cols = p.pair ? 256 : p.bn;
+  auto tiles = [&](int r, int c, int n) { return (long)((M + r - 1) / r) * ((n + c - 1) / c); };
+  auto pass = [&](double bytes, double tbs) { return 2.0 + 1e-6 * bytes / tbs * (double)M * ff; };
+  const double apart = PRODUCT[i8][form].us(tiles(rows, cols, 2 * ff), p.pair ? pairs : bb::sm_count(), nkb) + (i8 ? pass(5, 3.5) : pass(6, 5.0));
+  const double fused = PAIR_GLU[i8].us(tiles(256, 128, ff), pairs, nkb) + (i8 ? pass(3, 4.0) : 0.0);
+  return fused < apart;
+}
+
 // Slices of K for an accumulating GEMM of a given tile width: the count (<= 8, >= 16 k-blocks each) with the best wave efficiency.
 int pick_split(int M, int N, int nkb, int bn) {
   const long tiles = (long)((M + 127) / 128) * ((N + bn - 1) / bn);
@@ -983,6 +1013,8 @@ int pick_split(int M, int N, int nkb, int bn) {
   return pick;
 }
 }  // namespace
+
+BB_API int bb_glu_on_pairs(int i8, int M, int ff, int K) { return glu_on_pairs(i8 != 0, M, ff, K); }
 
 // C ABI ------------------------------------------------------------------------------------------
 // bf16 GEMM.  a_mn/b_mn: 0 = operand stored [rows][K] (K contiguous), 1 = stored [K][rows].

@@ -19,7 +19,6 @@
 // :1557-1623 (chunked prefill).
 #include <cmath>
 #include <cstdint>
-#include <cstdlib>
 
 #include "../common/host.hpp"
 
@@ -39,6 +38,7 @@ int bb_gemm_rows(const void* A, const void* B, void* C, const float* bias, const
                  int smem_kb, int early, void* stream);
 int bb_gemm_rows_glu(const void* A, const void* B, void* C, const float* bias, const float* scale_m, const float* scale_n,
                      int M, int ff, int K, int lda, int ldb, int ldc, int i8, int early, void* stream);
+int bb_glu_on_pairs(int i8, int M, int ff, int K);
 int bb_gemm_pair_glu(const void* A, const void* B, void* C, const float* scale_m, const float* scale_n, int M, int ff, int K,
                      int lda, int ldb, int ldc, void* stream);
 int bb_qk_rope_kv(const void* x, int ldx, const void* w_q, const void* w_k, const float* cos_t, const float* sin_t,
@@ -179,15 +179,6 @@ int linear(const BbLin& L, const void* x, int ldx, void* y, int rows, const BbSe
   return bb_gemm_bf16(x, L.w, y, L.bias, rows, L.n, L.k, ldx, L.k, L.n, 0, 0, 0, 1.0f, 0, 0, stream);
 }
 
-// BB_GEMM_PAIR=0 keeps every GEMM on one CTA a tile
-bool pair_gemms() {
-  static const bool on = [] {
-    const char* e = getenv("BB_GEMM_PAIR");
-    return !e || atoi(e) != 0;
-  }();
-  return on;
-}
-
 // Sum `x` [n elements] over the tensor-parallel group; returns where the result lives.
 int all_reduce(const BbServeCfg& c, BbServeState& s, void* x, long n, void** out, void* stream) {
   if (c.tp_world <= 1) {
@@ -241,7 +232,7 @@ int post_attn(const BbServeCfg& c, int li, const BbServeWork& w, int n, BbServeS
   if (i8 == q8 && L.gate_up.n == 2 * c.ff) {
     if (n < 256)
       act = bb_gemm_rows_glu(x, L.gate_up.w, w.act, L.gate_up.bias, sx, L.gate_up.scale, n, c.ff, k, k, k, c.ff, i8, 1, stream) == BB_OK;
-    else if (!L.gate_up.bias && pair_gemms())
+    else if (!L.gate_up.bias && bb_glu_on_pairs(i8, n, c.ff, k))
       act = bb_gemm_pair_glu(x, L.gate_up.w, w.act, sx, L.gate_up.scale, n, c.ff, k, k, k, c.ff, stream) == BB_OK;
   }
   bool down = false;

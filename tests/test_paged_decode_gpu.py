@@ -104,6 +104,20 @@ def _run(int8, tables, q, pools, scales, lens, hq, hk, hd, bs, splits):
     return out, po, pm
 
 
+@pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("hd,ratio,hk,bs,splits,times", [(128, 4, 2, 16, 8, 1), (128, 2, 2, 16, 9, 1), (64, 3, 2, 16, 16, 1), (128, 8, 1, 24, 16, 1),
+                                                         (128, 4, 4, 16, 3, 10), (64, 1, 4, 16, 3, 10)])
+def test_splits_in_clusters_and_behind_a_merge_kernel(hd, ratio, hk, bs, splits, times, int8):
+    """Eight splits are the last that merge in their cluster; more, or more than two CTAs an SM (here 840), leave parts to a
+    second kernel.  Sequences of fewer keys than splits among them."""
+    lens = LENS * times
+    hq = hk * ratio
+    _, tables, q, pools, scales, n, want = _case(hq, hk, hd, bs, int8, lens)
+    out, _, _ = _run(int8, tables, q, pools, scales, n, hq, hk, hd, bs, splits)
+    err = (out.double() - want).norm(dim=1) / want.norm(dim=1)
+    assert float(err.max()) < (2 ** -9 + 2e-3 if int8 else 2 ** -9 + 2 ** -14), err      # as above
+
+
 @pytest.mark.parametrize("hd,ratio", [(128, 1), (128, 2), (128, 4), (128, 8), (64, 1), (64, 2), (64, 3), (64, 4)])
 def test_weights_keep_their_24_bits(hd, ratio):
     """The fp32 parts, merged in 64 bits.  A weight is good to 2^-22 (two units of exp2, scores of size 1 summed in fp32) and

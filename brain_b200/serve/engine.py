@@ -299,7 +299,9 @@ class QwenEngine(PagedEngineBase):
 
     def _splits(self, B: int) -> int:
         """KV splits of the decode attention: enough CTAs to fill the machine (B * hk * splits >= ~4
-        per SM), and no more than merge in the kernel where contexts are short."""
+        per SM), and no more than merge in the kernel where contexts are short.  us a layer with 8 / 16
+        splits, one sequence, 4 kv heads: 700 keys 4.9 / 6.4, 2048 6.9 / 8.3, 4096 9.8 / 9.9 (8 kv heads of
+        4: 10.6 / 10.2); five to eight sequences of 8 kv heads at 4096 24 to 31 with 8, 24 to 35 with 10 to 15."""
         if self.decode_splits > 0:
             return self.decode_splits
         return max(1, min(8 if self.max_seq_len <= 4096 else 16, (4 * 148 + B * self.hk - 1) // (B * self.hk)))
@@ -592,9 +594,9 @@ class QwenEngine(PagedEngineBase):
         n = n_pre + B
         positions = np.asarray(positions, dtype=np.int32)
         block_tables = np.asarray(block_tables, dtype=np.int32)
+        self._check_positions(positions, block_tables)
         pos_np = [np.arange(it[1], it[1] + l, dtype=np.int32) for it, l in zip(items, lens)]
         # the rows that sample: last row of each finishing prompt + decode rows
-        self._check_positions(positions, block_tables)
         final = [i for i, it in enumerate(items) if it[3]]
         tok, pos, slots, dlens, rows, dbts, *bts = self._upload(
             np.concatenate([np.asarray(it[0], dtype=np.int32) for it in items] + [np.asarray(tokens, dtype=np.int32)]),
@@ -642,12 +644,12 @@ class QwenEngine(PagedEngineBase):
         a["decode_rows"] += B
         return results, [[int(p)] for p in picked[nf:]], (cands[nf:] if cands is not None else None)
 
-    def _decode_steps(self, tok, pos, bts, window: int, greedy: bool, slots=None):
-        """``window`` decode steps on device tensors -> (tokens [B, window], last top-k or None)."""
     def _decode(self, tokens, positions, block_tables, window, greedy, slots):
         self._check_positions(positions, block_tables, window)
         return super()._decode(tokens, positions, block_tables, window, greedy, slots)
 
+    def _decode_steps(self, tok, pos, bts, window: int, greedy: bool, slots=None):
+        """``window`` decode steps on device tensors -> (tokens [B, window], last top-k or None)."""
         B = tok.shape[0]
         outs = []
         topks = None

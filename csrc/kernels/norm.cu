@@ -504,7 +504,9 @@ __global__ void layernorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy,
 // Backward of a norm in one pass over its rows (d <= 1024): dx, and the sums over rows that are the gradients of gain (and
 // bias).  A warp walks its rows with the sums of its columns in registers, a block adds its warps' through shared memory and
 // adds the result to dw (db).  Apart, the sums read dy and x again, by two bytes a lane: us apart / here, RMSNorm 16384 x 1024
-// 47 / 27, LayerNorm 4096 x 768 14.9 / 8.1.  Bound by memory; wider rows do not leave the sums room in registers.
+// 47 / 27, LayerNorm 4096 x 768 14.9 / 8.1.  Bound by memory up to 768 columns; LayerNorm of 769 to 1024 spills (172 bytes a
+// thread at 128 registers) and gains less, 16384 x 1024 59 / 52 where its bytes take 21.  Wider rows do not leave the sums room
+// in registers.
 // LN: LayerNorm (mean, db), else RMSNorm.
 template <bool LN, int MAXV>
 __global__ void __launch_bounds__(256, 2)

@@ -4,8 +4,8 @@
 // Bound: HBM (every page row is read once).  The scalar form of this kernel (eight lanes per key, dot products and
 // P.V on the FMA pipe) was bound by instruction issue instead: 4 query heads per kv head cost 2 x 4 FMA per stored
 // element, plus conversions for int8 pages.  Measured for one layer, before -> after:
-//   bf16, 64 x 2050 keys, 4 kv heads, group of 4:   105.3 -> 49.8 us (268 MB, 5.4 TB/s)
-//   int8, 200 sequences of 128..2304 keys, 8 kv heads, group of 4:   333 -> 105 us (514 MB, 4.9 TB/s)
+//   bf16, 64 x 2050 keys, 4 kv heads, group of 4:   105.3 -> 49.8 us (268 MB, 5.4 TB/s; in one split 133 -> 45.5)
+//   int8, 200 sequences of 128..2304 keys, 8 kv heads, group of 4:   333 -> 102 us (514 MB, 5.0 TB/s)
 //
 // Tile: 16 keys.  S^T[16 keys, 8 columns] = K Q^T and O^T[HD, 8 columns] += V^T P^T, so the stored rows are the
 // 16-row operands as they lie in memory (V through transposing loads) and the query heads are the eight columns.
@@ -15,7 +15,7 @@
 // four heads take two products, eight take three.  The pieces' sums are added at the end.  The unit cuts its sums off, which
 // over a long row of tiles would drift: a tile's products are added up on their own.  Error of the fp32 result against 64 bits
 // 2e-8 to 2e-7, as with fp32 FMAs (pieces of 17 bits: 2.5e-7 to 6e-7); its cost, us of 200 int8 sequences as above with 1 / 2 /
-// 4 / 8 heads a key: 99.9 / 99.6 / 99.9 / 71 -> 97.6 / 96.2 / 103.5 / 76, none in bf16.
+// 4 / 8 heads a key: 100 / 99 / 100 / 71 -> 97 / 97 / 102 / 77, none in bf16.
 //
 // int8 pages: scores are exact integer products (mma .s8) with the query as two int8 terms per element,
 // q ~ qs (hi + lo / 128), 14 bits relative to the head's largest component.  Values become fp16 exactly (a byte under

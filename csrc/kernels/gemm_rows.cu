@@ -339,15 +339,36 @@ int run(const void* A, const void* B, Args a, int K, int lda, int ldb, int slice
   return a.ff ? launch<I8, true>(tm_w, tm_x, a, smem, stream) : launch<I8, false>(tm_w, tm_x, a, smem, stream);
 }
 
-// Whether this kernel is the faster one.  It re-reads the rows once per 128 channels; the tiles of gemm_tcgen05.cu walk
-// all of K in one CTA.  us here / there: 1 x 1024 x 3072 6.5 / 17.6; 64 x 2048 x 6144 12 / 31; 128 x 6144 x 4096 18.7 /
-// 23.2, but 64 x 32768 x 1024 19.3 / 17.7; 128 x 12288 x 2048 18.9 / 15.9; 200 x 24576 x 4096 67 / 62.  int8, whose other
-// kernel is slower still: 200 x 24576 x 4096 47 / 69; from 256 rows on the CTA-pair kernel takes 39.
-bool better(int M, int tiles, int nkb, bool i8) {
+// Whether this kernel is the faster one.  It re-reads the rows once per 128 channels and adds its slices up afterwards; the
+// tiles of gemm_tcgen05.cu walk all of K in one CTA, which takes long where K is long and is over at once where it is short.
+// The lines lie where measured sizes cross (8 to 255 rows, 384 to 151936 channels, K 64 to 12288): the form taken is 0.2 %
+// behind the faster one in the mean, by more than 8 % at 17 of 1400.  us here / there: 8 x 1024 x 1024 4.1 / 8.6, 48 x 1024 x 768
+// 5.2 / 7.5, 40 x 12288 x 256 9.0 / 6.3, 64 x 6144 x 2048 10.3 / 13.8, 128 x 6144 x 4096 17.6 / 22.5, 210 x 6144 x 2048 19.4 / 14.4,
+// 210 x 4096 x 4096 16.0 / 22.6, 224 x 4096 x 12288 32 / 60; int8 40 x 6144 x 1024 6.4 / 7.3, 128 x 1024 x 512 8.7 / 6.2, 160 x 6144
+// x 4096 14.3 / 15.3, 210 x 6144 x 4096 20.2 / 15.2, 255 x 1024 x 1024 13.7 / 7.3, 255 x 24576 x 4096 50 / 37.
+// In a step of dependent launches (early) this kernel's launch, prologue and first weights hide behind the kernel before it, and
+// the tiles' do not: about 4.5 us, which shift the lines.  us a decode step, lines of a lone product / these: int8 128 sequences
+// of width 4096 592 / 573, 96 of 2048 668 / 651; always this kernel / these: int8 200 (padded to 224) of width 1024 893 / 844, 210
+// of 2048 906 / 880.
+bool better(int M, int tiles, int nkb, bool i8, bool early) {
   if (M >= 256) return false;
-  if (i8 || M <= 48) return true;
-  if (M <= 64) return tiles <= 148 || nkb >= 32;
-  return (nkb >= 32 && tiles <= 48) || (nkb >= 64 && M <= 128);
+  if (M <= 32) return true;
+  const bool wide = tiles > 148;                            // more tiles than SMs: several CTAs of this kernel share one
+  if (early && M <= 224) {
+    if (i8) return M <= 112 || nkb >= (M <= 160 ? 6 : M <= 208 ? 16 : 32);
+    if (M <= 64) return M <= 48 || !wide || nkb >= 32;
+    if (tiles <= 48 && nkb >= (M <= 208 ? 32 : 64)) return true;
+  }
+  if (i8) {
+    if (M <= 64) return nkb >= 16 || (nkb >= 8 && tiles <= (M <= 48 ? 48 : 24)) || (wide && nkb >= (M <= 48 ? 3 : 6));
+    if (M <= 128) return nkb >= 16 && 2 * tiles <= (M <= 96 ? 6 : 3) * nkb;
+    if (M <= 160) return nkb >= 32 || (nkb >= 24 && tiles <= 32);
+    return nkb >= 24 && tiles <= (M <= 192 ? nkb : 3 * nkb / 4);
+  }
+  if (M <= 48) return nkb >= 12 || (nkb >= 8 && tiles <= 48) || (wide && nkb >= 6);
+  if (M <= 64) return (nkb >= 8 && tiles <= 48) || (nkb >= 12 && !wide) || nkb >= 32;
+  if (M <= 160) return (nkb >= 32 && tiles <= 48) || (nkb >= 64 && M <= 128);
+  return nkb >= 32 && (tiles <= 32 || 8 * tiles <= 3 * nkb);
 }
 
 // Slices of K and shared memory a CTA.  Many tiles: three CTAs an SM (74 KB hold two or three stages), one to four slices
@@ -401,7 +422,7 @@ static int gemm_rows(const void* A, const void* B, void* C, const float* bias, c
   a.err = device_error_word();
   if (slices == 0) {
     const int per = ff ? rows::BN / 2 : rows::BN, tiles = (N + per - 1) / per, nkb = (K + (i8 ? 127 : 63)) / (i8 ? 128 : 64);
-    if (!rows::better(M, tiles, nkb, i8)) return BB_ESIZE;
+    if (!rows::better(M, tiles, nkb, i8, early)) return BB_ESIZE;
     rows::split(M, tiles, nkb, sm_count(), &slices, &smem_kb);
   }
   if (slices < 1 || slices > 8 || smem_kb < 32 || smem_kb > 226) return BB_EARG;

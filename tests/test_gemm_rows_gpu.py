@@ -63,6 +63,25 @@ def test_int8(M, N, K):
     assert bool((err <= 2 ** -8 * 1.01 * want.abs()).all()), float(err.max())
 
 
+@pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("slices,smem_kb", [(1, 74), (4, 110), (8, 220)])
+@pytest.mark.parametrize("M,N,K", SIZES)
+def test_splits_that_the_choice_by_size_leaves_out(M, N, K, slices, smem_kb, int8):
+    """Every size under given slices of K, also where the general call takes another kernel; sums of whole numbers are exact."""
+    g = torch.Generator("cuda").manual_seed(M + N + K)
+    K = -(-K // 16) * 16
+    a, b = (torch.randint(-8, 9, (r, K), device="cuda", dtype=torch.int8, generator=g) for r in (M, N))
+    one = torch.ones(max(M, N), device="cuda")
+    x, w = (a, b) if int8 else (a.bfloat16(), b.bfloat16())
+    out = torch.full((M, N), 7.0, device="cuda", dtype=torch.bfloat16 if int8 else torch.float32)
+    rc = _cuda.lib().bb_gemm_rows(_p(x), _p(w), _p(out), _p(None), _p(one if int8 else None), _p(one if int8 else None), M, N, K, K, K, N,
+                                  int(int8), 0 if int8 else 1, C.c_float(1.0), slices, smem_kb, 0, _stream())
+    assert rc == 0
+    _cuda.check_error()
+    want = a.double() @ b.double().t()                                        # below 2^24: exact in fp32
+    assert torch.equal(out, want.to(out.dtype))
+
+
 def test_same_sum_every_run():
     a = torch.randn(33, 4096, device="cuda").bfloat16()
     b = torch.randn(1024, 4096, device="cuda").bfloat16()

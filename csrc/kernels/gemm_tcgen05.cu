@@ -928,11 +928,13 @@ namespace {
 // us of `tiles` tiles over `slots` CTAs (or pairs), every tile nkb k-blocks of 128 bytes: whole waves, and the first fill and
 // last epilogue of the launch.  The per-block and fixed times are fits to measured launches (2048 to 4593 rows, 6 to 2374
 // blocks), good to about 10 %; what matters is the order of the forms.
+// Where 64 and 128 columns come out alike over one long K, 64 it is: rows that do not start on 128 bytes cost the wider tile more
+// (324 x 3072 x 10280 70 us / 86, 1194 x 824 x 8504 52 / 61; of 10240 and 8512 both take the same).
 struct GemmForm {
   int bn;                // 0: CTA pairs, 256 x 256
   double per_block, fixed;
 };
-constexpr GemmForm FORMS[2][4] = {{{64, 0.31, 4.0}, {128, 0.30, 5.2}, {256, 0.40, 5.2}, {0, 0.36, 6.0}},     // bf16
+constexpr GemmForm FORMS[2][4] = {{{64, 0.31, 4.0}, {128, 0.305, 5.2}, {256, 0.40, 5.2}, {0, 0.36, 6.0}},     // bf16
                                   {{64, 0.27, 4.5}, {128, 0.29, 5.0}, {256, 0.41, 5.0}, {0, 0.38, 6.0}}};   // int8
 
 struct GemmPick {
